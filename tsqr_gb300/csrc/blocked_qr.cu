@@ -999,7 +999,7 @@ constexpr int kHrMax = 32;  // panel width limit of the Householder path
 // Reconstruction of one panel, one CTA.  In: the top bw x bw block of the
 // panel's explicit Q (at Ap, lda) and its TSQR factor Rp (bw x bw, ldrp).
 // Out: the top block rewritten as the unit lower triangular Y_1, U^-1
-// (ld kHrMax), T (bw x bw at Tp, ld ldt), R_h = S Rp into Rout (upper
+// (bw x bw, ld bw: its workspace block has b * b elements), T (bw x bw at Tp, ld ldt), R_h = S Rp into Rout (upper
 // triangle, ldr), and M = T Y_1^T = -U S, whose diagonal is T's, transposed
 // in the strict lower triangle of T's block (which no product reads).
 //
@@ -1067,7 +1067,7 @@ __global__ void __launch_bounds__(256) hr_reconstruct(int bw, T* Ap, int64_t lda
 #pragma unroll
             for (int k = 0; k < i; ++k)
                 if (i <= lane) x[k] = fma(-Wt[i][k], x[i], x[k]);
-            if (i < bw && lane < bw) Uinv[i + lane * kHrMax] = x[i];
+            if (i < bw && lane < bw) Uinv[i + lane * bw] = x[i];
         }
         return;
     }
@@ -1102,7 +1102,7 @@ __global__ void __launch_bounds__(256) hr_reconstruct(int bw, T* Ap, int64_t lda
     }
 }
 
-// Y <- Y U (kUinv: U at ld kHrMax, in place for the rows below a panel's top
+// Y <- Y U (kUinv: U = U^-1 of the panel, in place for the rows below a panel's top
 // block) or [I; 0] - Y M (the panel's columns of Q; M as hr_reconstruct leaves
 // it in T's block), U and M upper triangular, one thread per row.  The matrix
 // is read as 16-byte rows of four columns for kUpperRows rows at once: 144
@@ -1339,8 +1339,8 @@ tsqr_status hqr_factor(const HqrCtx<T>& c, int64_t m, int64_t n, T* A, T* Rb, T*
                    c.ldr);
         log_launch(kTagHouse, c.s);
         if (m > n) {
-            launch_pdl(rows_times_upper<T, true>, dim3((unsigned)ceil_div(m - n, 128 * kUpperRows<T>)), dim3(128), 0, c.s, m - n, (int)n,
-                       A + n, c.lda, c.Uinv, (int64_t)kHrMax);
+            launch_pdl(rows_times_upper<T, true>, dim3((unsigned)ceil_div(m - n, 128 * kUpperRows<T>)), dim3(128), 0,
+                       c.s, m - n, (int)n, A + n, c.lda, c.Uinv, n);
             log_launch(kTagHouse + 1, c.s);
         }
         return TSQR_OK;
