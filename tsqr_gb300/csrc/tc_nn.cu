@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (lane == 0) {  // MMAs
         constexpr uint32_t idesc = tc::idesc_tf32(128, NB);
         const uint32_t sh = tc::smem_u32(bhi), so = tc::smem_u32(blo);
-        int t = 0;
-        for (int j = 0, s = 0; t < T; ++t) {
+        int t = 0, j = 0;
+        for (int s = 0; t < T; ++t) {
             const int sl = t % kSlots, b = j & 1;
             if (s == 0 && j >= 2 &&
                 !tc::mbar_wait(tc::smem_u32(&dempty[b]), (uint32_t)(j / 2 - 1) & 1u, tries))
@@ -251,6 +251,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (t < T && err) atomicExch(err, 1);
         for (int q = max(0, t - kSlots); q < t; ++q)  // every MMA is done
             (void)tc::mbar_wait(tc::smem_u32(&done[q % kSlots]), (uint32_t)(q / kSlots) & 1u);
+        // and so is the arrival for every finished block: the warps that add
+        // it to C may have given up, and it must not come after the CTA's end
+        for (int q = max(0, j - 2); q < j; ++q)
+            (void)tc::mbar_wait(tc::smem_u32(&dfull[q & 1]), (uint32_t)(q >> 1) & 1u);
     }
     __syncwarp();
     tc::fence_before_sync();
