@@ -69,14 +69,15 @@ tsqr_status tsqr_ex(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, 
     f.norm64 = o.fp64_scalars != 0;
     f.root64 = o.fp64_root != 0;
     // one TSQR pass of the chosen form over A, its R to Rp; a second pass
-    // keeps the first pass's tensor-core status
+    // keeps the first pass's report in the status word
     auto pass = [&](T* Rp, int64_t ldrp, size_t bytes, bool first) -> tsqr_status {
+        int* status = first ? nullptr : reinterpret_cast<int*>(work);
         if (prec) {
-            f.clear_status = first;
+            f.status = status;
             return tsqr::tsqr_precision(m, n, reinterpret_cast<float*>(A), lda, reinterpret_cast<float*>(Rp), ldrp,
                                         work, bytes, s, f);
         }
-        return tsqr::tsqr_plain<T>(m, n, A, lda, Rp, ldrp, work, bytes, s);
+        return tsqr::tsqr_plain<T>(m, n, A, lda, Rp, ldrp, work, bytes, s, tsqr::kPhaseUp | tsqr::kPhaseDown, status);
     };
     if (!o.reorth) return pass(R, ldr, work_bytes, true);
     // one reorthogonalisation pass: Q1 R1 = A, then Q2 R2 = Q1, so that

@@ -922,25 +922,35 @@ tsqr_status proj_tn(int64_t m, int64_t n1, int64_t n2, const T* A1, const T* A2,
 }
 
 
+// TSQR of one panel in the call's form, its bounded waits reporting to the
+// call's status word.
+template <typename T>
+tsqr_status panel_tsqr(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, void* work, size_t work_bytes,
+                       bool tc, int* status, cudaStream_t s) {
+    if constexpr (std::is_same<T, float>::value) {
+        if (tc) {
+            PrecFlags f;
+            f.status = status;
+            return tsqr_precision(m, n, A, lda, R, ldr, work, work_bytes, s, f);
+        }
+    }
+    return tsqr_plain<T>(m, n, A, lda, R, ldr, work, work_bytes, s, kPhaseUp | kPhaseDown, status);
+}
+
 template <typename T>
 tsqr_status qr_rec(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, char* ws, const QrWs& w,
                    const tsqr_opts& o, cudaStream_t s) {
     const int nb = panel_of(o);
     const bool tc = use_tc<T>(o);
     char* tws = ws + w.err_bytes;
-    if (n <= nb) {
-        if constexpr (std::is_same<T, float>::value) {
-            if (tc) return tsqr_precision(m, n, A, lda, R, ldr, tws, w.tsqr_bytes, s);
-        }
-        return tsqr_plain<T>(m, n, A, lda, R, ldr, tws, w.tsqr_bytes, s);
-    }
+    int* err = reinterpret_cast<int*>(ws);
+    if (n <= nb) return panel_tsqr<T>(m, n, A, lda, R, ldr, tws, w.tsqr_bytes, tc, err, s);
     const int64_t n1 = split_of(n, nb), n2 = n - n1;
     T* A1 = A;
     T* A2 = A + n1 * lda;
     T* R11 = R;
     T* R12 = R + n1 * ldr;
     T* R22 = R + n1 * ldr + n1;
-    int* err = reinterpret_cast<int*>(ws);
     int* cnt = err + kPCounters;
     T* P = reinterpret_cast<T*>(tws + w.tsqr_bytes);
     T* tmp = reinterpret_cast<T*>(tws + w.tsqr_bytes + w.part_bytes);
@@ -1327,13 +1337,7 @@ void hqr_nn(const HqrCtx<T>& c, int64_t m, int64_t n1, int64_t n2, const T* Y, c
 template <typename T>
 tsqr_status hqr_factor(const HqrCtx<T>& c, int64_t m, int64_t n, T* A, T* Rb, T* Tb) {
     if (n <= c.b) {
-        tsqr_status st;
-        if constexpr (std::is_same<T, float>::value) {
-            st = c.tc ? tsqr_precision(m, n, A, c.lda, c.Rp, n, c.tws, c.tsqr_bytes, c.s)
-                      : tsqr_plain<T>(m, n, A, c.lda, c.Rp, n, c.tws, c.tsqr_bytes, c.s);
-        } else {
-            st = tsqr_plain<T>(m, n, A, c.lda, c.Rp, n, c.tws, c.tsqr_bytes, c.s);
-        }
+        tsqr_status st = panel_tsqr<T>(m, n, A, c.lda, c.Rp, n, c.tws, c.tsqr_bytes, c.tc, c.err, c.s);
         if (st != TSQR_OK) return st;
         launch_pdl(hr_reconstruct<T>, dim3(1), dim3(256), 0, c.s, (int)n, A, c.lda, c.Rp, (int)n, c.Uinv, Tb, c.ldt, Rb,
                    c.ldr);

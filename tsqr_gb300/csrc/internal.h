@@ -152,13 +152,15 @@ enum { kTagFactor = 1000, kTagApply = 2000, kTagGemmTN = 3000, kTagReduce = 4000
 
 // Plain-precision TSQR tree (tsqr.cu).  phases: the up-sweep (factor every
 // level, R out) and / or the down-sweep (explicit Q from the compact-WY
-// tree left in A and the workspace by the up-sweep).
+// tree left in A and the workspace by the up-sweep).  status: the word that
+// bounded waits report to, zeroed by the caller (a pass inside a larger call);
+// null: the word at the start of work, zeroed by the up-sweep.
 enum { kPhaseUp = 1, kPhaseDown = 2 };
 template <typename T>
 size_t tsqr_plain_workspace(int64_t m, int64_t n);
 template <typename T>
 tsqr_status tsqr_plain(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, void* work, size_t work_bytes,
-                       cudaStream_t s, int phases = kPhaseUp | kPhaseDown);
+                       cudaStream_t s, int phases = kPhaseUp | kPhaseDown, int* status = nullptr);
 // One level of the tree as the up-sweep leaves it: h rows (column-major, ld)
 // cut into ntiles tiles of `rows` rows, each holding V below its diagonal
 // and T in its top block's upper triangle; level 0 is A, the last level is
@@ -194,12 +196,11 @@ namespace tsqr {
 // Precision form of TSQR (tsqr.cu + tc_apply.cu), FP32 only.  Options:
 // norm64 -- per-column norm, beta and tau in FP64 (tsqr_opts.fp64_scalars);
 // root64 -- root combine in FP64, n <= 32 (tsqr_opts.fp64_root);
-// clear_status -- zero the status word first (off for a second pass that
-// must keep the first pass's report).
+// status -- as for tsqr_plain.
 struct PrecFlags {
     bool norm64 = false;
     bool root64 = false;
-    bool clear_status = true;
+    int* status = nullptr;
 };
 size_t tsqr_precision_workspace(int64_t m, int64_t n, PrecFlags f = PrecFlags());
 // TSQR of host-resident A with host Q and R, transfers pipelined with the

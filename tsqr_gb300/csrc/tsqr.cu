@@ -300,7 +300,7 @@ size_t tsqr_plain_workspace(int64_t m, int64_t n) {
 
 template <typename T>
 tsqr_status tsqr_plain(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, void* work, size_t work_bytes,
-                       cudaStream_t s, int phases) {
+                       cudaStream_t s, int phases, int* status) {
     KernelSet<T> ks = pick((T*)nullptr, (int)n);
     if (!ks.factor) return TSQR_ERR_UNSUPPORTED;
     std::vector<Level<T>> lv;
@@ -309,7 +309,8 @@ tsqr_status tsqr_plain(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ld
     if (need > 0 && (work == nullptr || work_bytes < kAlign + need)) return TSQR_ERR_WORKSPACE;
     // a single-tile problem may run without a workspace, and then without a
     // status word
-    int* err = (work != nullptr && work_bytes >= kAlign) ? reinterpret_cast<int*>(work) : nullptr;
+    int* err = status;
+    if (!err && work != nullptr && work_bytes >= kAlign) err = reinterpret_cast<int*>(work);
     const int L = (int)lv.size();
     // up-sweep
     for (int l = 0; l < L && (phases & kPhaseUp); ++l) {
@@ -321,7 +322,7 @@ tsqr_status tsqr_plain(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ld
         fp.ntiles = lv[l].ntiles;
         fp.stack = l > 0;
         fp.err = err;
-        fp.clear = l == 0 ? err : nullptr;
+        fp.clear = l == 0 && !status ? err : nullptr;
         fp.tries = wait_tries().load(std::memory_order_relaxed);
         if (l == L - 1) {
             fp.Rout = R;
@@ -462,13 +463,13 @@ tsqr_status tsqr_precision(int64_t m, int64_t n, float* A, int64_t lda, float* R
     const PrecLayout PL = prec_layout(m, n, c, f.root64);
     if (work == nullptr || work_bytes < PL.total) return TSQR_ERR_WORKSPACE;
     char* base = reinterpret_cast<char*>(work);
-    int* err = reinterpret_cast<int*>(base + PL.status);
+    int* err = f.status ? f.status : reinterpret_cast<int*>(base + PL.status);
     std::vector<Level<float>> lv;
     plan_levels<float>(m, n, A, lda, c.rows, base + PL.levels, &lv);
     const int L = (int)lv.size();
     const bool root64 = f.root64;
     const int top = root64 ? L - 1 : L;  // levels factored in FP32 below the root
-    if (f.clear_status && top == 0 && cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return TSQR_ERR_CUDA;
+    if (!f.status && top == 0 && cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return TSQR_ERR_CUDA;
     for (int l = 0; l < top; ++l) {
         FactorParams<float> fp;
         fp.M = lv[l].M;
@@ -478,7 +479,7 @@ tsqr_status tsqr_precision(int64_t m, int64_t n, float* A, int64_t lda, float* R
         fp.ntiles = lv[l].ntiles;
         fp.stack = l > 0;
         fp.err = err;
-        fp.clear = l == 0 && f.clear_status ? err : nullptr;
+        fp.clear = l == 0 && !f.status ? err : nullptr;
         fp.tries = wait_tries().load(std::memory_order_relaxed);
         fp.Rout = (l == L - 1) ? R : lv[l + 1].M;
         fp.ldr = (l == L - 1) ? ldr : lv[l + 1].ld;
@@ -540,9 +541,9 @@ template tsqr_status tsqr_plain_tree<float>(int64_t, int64_t, const float*, int6
 template tsqr_status tsqr_plain_tree<double>(int64_t, int64_t, const double*, int64_t, const void*, size_t,
                                              std::vector<TreeLevel<double>>*);
 template tsqr_status tsqr_plain<float>(int64_t, int64_t, float*, int64_t, float*, int64_t, void*, size_t,
-                                       cudaStream_t, int);
+                                       cudaStream_t, int, int*);
 template tsqr_status tsqr_plain<double>(int64_t, int64_t, double*, int64_t, double*, int64_t, void*, size_t,
-                                        cudaStream_t, int);
+                                        cudaStream_t, int, int*);
 
 // ---------------------------------------------------------------------------
 // TSQR of a matrix in host memory (tsqr_s_host / tsqr_d_host).  The device
