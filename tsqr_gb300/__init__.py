@@ -369,7 +369,8 @@ def qr_(A, R=None, precision="plain", reorth=False, panel=0, work=None, stream=N
     nbytes = int(lib().qr_workspace_bytes(m, n, A.element_size(), ctypes.byref(o)))
     if nbytes == 0:
         raise TsqrError(2, "qr_ workspace (m=%d n=%d)" % (m, n))
-    w, wb = _work(nbytes, work, A.device)
+    # a caller's buffer may be smaller than the query's answer (FP64); the library says whether it is enough
+    w, wb = _work(nbytes if work is None else 0, work, A.device)
     fn = lib().qr_s_ex if A.dtype == torch.float32 else lib().qr_d_ex
     _check(fn(m, n, A.data_ptr(), lda, R.data_ptr(), ldr, w.data_ptr(), wb, ctypes.byref(o),
               _stream_handle(stream)), "qr_")
@@ -388,7 +389,7 @@ def profile_(kind, A, R, precision="plain", reorth=False, panel=0, work=None, st
     k = 0 if kind == "tsqr" else 1
     nbytes = (lib().tsqr_workspace_bytes if k == 0 else lib().qr_workspace_bytes)(m, n, A.element_size(),
                                                                                  ctypes.byref(o))
-    w, wb = _work(int(nbytes), work, A.device)
+    w, wb = _work(int(nbytes) if work is None else 0, work, A.device)
     ms = (ctypes.c_float * max_launch)()
     tags = (ctypes.c_int * max_launch)()
     cnt = ctypes.c_int(0)

@@ -721,30 +721,50 @@ struct GemmPlan {
     int64_t kchunk;
 };
 
-GemmPlan tn_plan(int64_t M, int64_t N, int64_t K) {
+// At most most_nz chunks (the room for partial sums).
+GemmPlan tn_plan(int64_t M, int64_t N, int64_t K, int64_t most_nz = INT32_MAX) {
     // two CTAs per SM of GB300's 152 (the workspace query uses the same plan),
     // chunks of 64 rows or more
     const int64_t tiles = ceil_div(M, kTnTile) * ceil_div(N, kTnTile);
     int64_t nz = std::max<int64_t>(1, (2 * 152) / tiles);
     nz = std::min<int64_t>(nz, std::max<int64_t>(1, ceil_div(K, 64)));
+    nz = std::min<int64_t>(nz, most_nz);
     int64_t kchunk = round_up(ceil_div(K, nz), kKt);
     nz = ceil_div(K, kchunk);
     return {(int)nz, kchunk};
 }
 
-// Bytes of partial sums proj_tn needs for an n1 x n2 projection over K rows.
+// Bytes of partial sums proj_tn takes for an n1 x n2 projection over K rows.
 template <typename T>
 size_t proj_tn_part_bytes(int64_t n1, int64_t n2, int64_t K) {
     if (std::is_same<T, float>::value) return tn_fused_plan(n1, n2, K).part_bytes();
     return (size_t)tn_plan(n1, n2, K).nz * n1 * n2 * sizeof(T);
 }
 
+// Bytes it can do with: FP64 takes fewer and longer chunks where the room is
+// short.  The least is what the query asked for with 64-wide tiles in chunks
+// of 256 rows, so that a buffer of that size stays enough.
+template <typename T>
+size_t proj_tn_part_least(int64_t n1, int64_t n2, int64_t K) {
+    const size_t want = proj_tn_part_bytes<T>(n1, n2, K);
+    if (std::is_same<T, float>::value) return want;
+    const int64_t nz = std::min<int64_t>(ceil_div(2 * 152, ceil_div(n1, 64) * ceil_div(n2, 64)), ceil_div(K, 256));
+    return std::min(want, (size_t)(ceil_div(K, round_up(ceil_div(K, nz), kKt)) * n1 * n2) * sizeof(T));
+}
+
+// Room for partial sums in a workspace of `have` bytes that needs `least`
+// with `part_least` of them: more where there is more, up to `want`.
+size_t part_room(size_t have, size_t least, size_t part_least, size_t want) {
+    return std::min(want, part_least + (have - least) / 256 * 256);
+}
+
 // Workspace layout: [status word | tsqr region | partial sums | reorth temp].
 // The precision form (FP32, TF32X3) sizes the TSQR region for the
 // precision-form TSQR and the partial sums for the tcgen05 split-K GEMM.
 struct QrWs {
-    size_t err_bytes = kPHeader, tsqr_bytes = 0, part_bytes = 0, tmp_bytes = 0;
+    size_t err_bytes = kPHeader, tsqr_bytes = 0, part_bytes = 0, part_least = 0, tmp_bytes = 0;
     size_t total() const { return err_bytes + tsqr_bytes + part_bytes + tmp_bytes; }
+    size_t least() const { return total() - part_bytes + part_least; }
 };
 
 // The tensor-core forms (FP32 only): TF32X3, or BF16X3, whose GEMMs use
@@ -775,7 +795,9 @@ void qr_ws_walk(int64_t m, int64_t n, int nb, bool reorth, bool tc, QrWs* w) {
     const int64_t n1 = split_of(n, nb), n2 = n - n1;
     const size_t pb = tc_projection(tc, n1, n2) ? (size_t)tc_tn_splits(n1, n2, m) * n1 * n2 * sizeof(T)
                                                 : proj_tn_part_bytes<T>(n1, n2, m);
+    const size_t pl = tc_projection(tc, n1, n2) ? pb : proj_tn_part_least<T>(n1, n2, m);
     w->part_bytes = std::max(w->part_bytes, (size_t)round_up((int64_t)pb, 256));
+    w->part_least = std::max(w->part_least, (size_t)round_up((int64_t)pl, 256));
     if (reorth) w->tmp_bytes = std::max(w->tmp_bytes, (size_t)round_up(n1 * n2 * (int64_t)sizeof(T), 256));
     qr_ws_walk<T>(m, n1, nb, reorth, tc, w);
     qr_ws_walk<T>(m, n2, nb, reorth, tc, w);
@@ -861,10 +883,10 @@ void update_nn(int64_t m, int64_t n1, int64_t n2, const T* A1, int64_t lda, cons
 // C (n1 x n2, ldc) = A1^T A2 (+ beta C) on CUDA cores.  FP32: one launch of
 // gemm_tn_fused (cnt: the workspace's counter words, zero between
 // launches), which adds the product to D as well if it is given; FP64: split-K
-// partials, then their sum (D must be null).
+// partials (part_bytes at P), then their sum (D must be null).
 template <typename T>
-tsqr_status proj_tn(int64_t m, int64_t n1, int64_t n2, const T* A1, const T* A2, int64_t lda, T* P, T* C,
-                    int64_t ldc, T beta, int* cnt, int* err, cudaStream_t s, T* D = nullptr, int64_t ldd = 0) {
+tsqr_status proj_tn(int64_t m, int64_t n1, int64_t n2, const T* A1, const T* A2, int64_t lda, T* P, size_t part_bytes,
+                    T* C, int64_t ldc, T beta, int* cnt, int* err, cudaStream_t s, T* D = nullptr, int64_t ldd = 0) {
     if constexpr (std::is_same<T, float>::value) {
         const TnFusedPlan fp = tn_fused_plan(n1, n2, m);
         TnFusedArgs a;
@@ -911,7 +933,7 @@ tsqr_status proj_tn(int64_t m, int64_t n1, int64_t n2, const T* A1, const T* A2,
         log_launch(kTagGemmTN, s);
         return TSQR_OK;
     }
-    GemmPlan gp = tn_plan(n1, n2, m);
+    GemmPlan gp = tn_plan(n1, n2, m, (int64_t)(part_bytes / (sizeof(T) * n1 * n2)));
     dim3 g((unsigned)ceil_div(n1, kTnTile), (unsigned)ceil_div(n2, kTnTile), (unsigned)gp.nz);
     launch_pdl(gemm_tn_partial<T>, g, dim3(256), 0, s, (int)n1, (int)n2, m, A1, lda, A2, lda, P, gp.kchunk);
     log_launch(kTagGemmTN, s);
@@ -961,10 +983,10 @@ tsqr_status qr_rec(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, c
         if (tcp)
             proj_tn_tc<T>(m, n1, n2, A1, A2, lda, P, R12, ldr, T(0), err, s, use_bf16<T>(o));
         else
-            proj_tn<T>(m, n1, n2, A1, A2, lda, P, R12, ldr, T(0), cnt, err, s);
+            proj_tn<T>(m, n1, n2, A1, A2, lda, P, w.part_bytes, R12, ldr, T(0), cnt, err, s);
         update_nn_tc<T>(m, n1, n2, A1, lda, R12, ldr, A2, err, s, use_bf16<T>(o));
     } else {
-        proj_tn<T>(m, n1, n2, A1, A2, lda, P, R12, ldr, T(0), cnt, err, s);
+        proj_tn<T>(m, n1, n2, A1, A2, lda, P, w.part_bytes, R12, ldr, T(0), cnt, err, s);
         update_nn<T>(m, n1, n2, A1, lda, R12, ldr, A2, s);
     }
     if (o.reorth) {
@@ -974,7 +996,7 @@ tsqr_status qr_rec(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, c
         if (tcp)
             proj_tn_tc<T>(m, n1, n2, A1, A2, lda, P, tmp, n1, T(0), err, s, use_bf16<T>(o));
         else
-            proj_tn<T>(m, n1, n2, A1, A2, lda, P, tmp, n1, T(0), cnt, err, s, D, ldr);
+            proj_tn<T>(m, n1, n2, A1, A2, lda, P, w.part_bytes, tmp, n1, T(0), cnt, err, s, D, ldr);
         if (tc)
             update_nn_tc<T>(m, n1, n2, A1, lda, tmp, n1, A2, err, s, use_bf16<T>(o));
         else
@@ -1261,8 +1283,9 @@ __global__ void __launch_bounds__(256) move_block(int n1, int64_t total, T* A, i
 // Workspace: [status word | leaf TSQR | split-K partials | Rp and U^-1 of a
 // leaf | W, X (n1 x n2 each) | T of the whole matrix (n x n)].
 struct HqrWs {
-    size_t err = kPHeader, tsqr = 0, part = 0, small = 0, wx = 0, tfull = 0;
+    size_t err = kPHeader, tsqr = 0, part = 0, part_least = 0, small = 0, wx = 0, tfull = 0;
     size_t total() const { return err + tsqr + part + small + wx + tfull; }
+    size_t least() const { return total() - part + part_least; }
 };
 
 template <typename T>
@@ -1276,7 +1299,9 @@ void hqr_ws_walk(int64_t m, int64_t n, int b, bool tc, HqrWs* w) {
     for (int64_t K : {m, m - n1}) {
         const size_t pb = tc_projection(tc, n1, n2) ? (size_t)tc_tn_splits(n1, n2, K) * n1 * n2 * sizeof(T)
                                                     : proj_tn_part_bytes<T>(n1, n2, K);
+        const size_t pl = tc_projection(tc, n1, n2) ? pb : proj_tn_part_least<T>(n1, n2, K);
         w->part = std::max(w->part, (size_t)round_up((int64_t)pb, 256));
+        w->part_least = std::max(w->part_least, (size_t)round_up((int64_t)pl, 256));
     }
     w->wx = std::max(w->wx, 2 * (size_t)round_up(n1 * n2 * (int64_t)sizeof(T), 256));
     hqr_ws_walk<T>(m, n1, b, tc, w);
@@ -1296,7 +1321,7 @@ template <typename T>
 struct HqrCtx {
     int64_t lda, ldr, ldt;
     char* tws;
-    size_t tsqr_bytes;
+    size_t tsqr_bytes, part_bytes;
     T *part, *Rp, *Uinv, *W, *X;
     int* err;
     bool tc;
@@ -1319,7 +1344,7 @@ void hqr_tn(const HqrCtx<T>& c, int64_t m, int64_t n1, int64_t n2, const T* A1, 
     if (tc_projection(c.tc, n1, n2))
         proj_tn_tc<T>(m, n1, n2, A1, A2, c.lda, c.part, C, n1, T(0), c.err, c.s, c.bf16);
     else
-        proj_tn<T>(m, n1, n2, A1, A2, c.lda, c.part, C, n1, T(0), c.err + kPCounters, c.err, c.s);
+        proj_tn<T>(m, n1, n2, A1, A2, c.lda, c.part, c.part_bytes, C, n1, T(0), c.err + kPCounters, c.err, c.s);
 }
 
 // A2 (m x n2) -= Y (m x n1) X (n1 x n2, ld n1)
@@ -1399,8 +1424,9 @@ tsqr_status hqr_run(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, 
     const int b = panel_of(o);
     if (b > kHrMax) return TSQR_ERR_UNSUPPORTED;
     const bool tc = use_tc<T>(o);
-    const HqrWs w = hqr_ws<T>(m, n, b, tc);
-    if (work == nullptr || work_bytes < w.total()) return TSQR_ERR_WORKSPACE;
+    HqrWs w = hqr_ws<T>(m, n, b, tc);
+    if (work == nullptr || work_bytes < w.least()) return TSQR_ERR_WORKSPACE;
+    w.part = part_room(work_bytes, w.least(), w.part_least, w.part);
     char* base = static_cast<char*>(work);
     HqrCtx<T> c;
     c.lda = lda;
@@ -1410,6 +1436,7 @@ tsqr_status hqr_run(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, 
     c.tws = base + w.err;
     c.tsqr_bytes = w.tsqr;
     c.part = reinterpret_cast<T*>(c.tws + w.tsqr);
+    c.part_bytes = w.part;
     const size_t bb = (size_t)round_up((int64_t)(b * b * sizeof(T)), 256);
     char* sm = c.tws + w.tsqr + w.part;
     c.Rp = reinterpret_cast<T*>(sm);
@@ -1446,7 +1473,8 @@ tsqr_status qr_run(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ldr, v
     if (o.algorithm == TSQR_QR_HOUSEHOLDER) return hqr_run<T>(m, n, A, lda, R, ldr, work, work_bytes, o, s);
     QrWs w;
     qr_ws_walk<T>(m, n, panel_of(o), o.reorth != 0, use_tc<T>(o), &w);
-    if (work == nullptr || work_bytes < w.total()) return TSQR_ERR_WORKSPACE;
+    if (work == nullptr || work_bytes < w.least()) return TSQR_ERR_WORKSPACE;
+    w.part_bytes = part_room(work_bytes, w.least(), w.part_least, w.part_bytes);
     // status word and the projection's counters
     if (cudaMemsetAsync(work, 0, kPHeader, s) != cudaSuccess) return TSQR_ERR_CUDA;
     // zeros below R's diagonal blocks, in one fill for all nodes
