@@ -254,12 +254,17 @@ __global__ void __launch_bounds__(kNT) apply_qt_column(QtParams<T, NMAX> p, int6
         }
         __syncthreads();
         // Z = T^T Y, then the top n rows of c - V Z
+        // FP64 stops past n: a predicated-off FP64 instruction costs its time. In
+        // steps of 8, whose loads stay in flight together
+        const int last = sizeof(T) == 8 ? n : NMAX;
         if (tid < n) {
             const int j = tid;
             T z = T(0);
 #pragma unroll
-            for (int i = 0; i < NMAX; ++i)
+            for (int i = 0; i < NMAX; ++i) {
+                if (i % 8 == 0 && i >= last) break;
                 if (i <= j) z = fma(W[j][i], yv[i], z);
+            }
             zv[j] = z;
         }
         __syncthreads();
@@ -267,8 +272,10 @@ __global__ void __launch_bounds__(kNT) apply_qt_column(QtParams<T, NMAX> p, int6
             const int j = tid;
             T v = cs[j] - zv[j];
 #pragma unroll
-            for (int i = 0; i < NMAX - 1; ++i)
+            for (int i = 0; i < NMAX - 1; ++i) {
+                if (i % 8 == 0 && i >= last) break;
                 if (i < j) v = fma(-W[i][j], zv[i], v);
+            }
             p.out[t * n + j + col * p.ldo] = v;
         }
         __syncthreads();  // the shared buffers are reused by the next tile
