@@ -433,20 +433,28 @@ PrecLayout prec_layout(int64_t m, int64_t n, const PrecCfg& c, bool root64_opt =
 
 bool tc_apply_level(const ApplyParams<float>& p, int nmax, int rows, int* err, cudaStream_t s);
 
-// Whether a level of the precision form takes the FP32 Q assembly.  Its CTA has
-// no TMEM to allocate, no operands to split and no padded columns to multiply.
-//   up to 32 columns, up to 128 tiles: yes.  us of one level at 32 columns,
-//     FP32 / tcgen05: 1 tile 6.5 / 11.4, 16 tiles 9.4 / 11.8; a whole call of
-//     65,536 x 32 (128, 8 and 1 tiles) 99 / 104;
-//   above that, 32 columns: no (4,194,304 x 32 956 / 943); fewer, where FP32
-//     copies 16 bytes at a time: yes (x 31 951 / 990, x 24 792 / 856, x 16
-//     324 / 339, 1,000,000 x 29 286 / 298), else no (2,243,789 x 29 583 / 573);
-//   33 to 64 columns: above 128 tiles (1,000,003 x 50 968 / 1013, 2,000,000 x 33
-//     1202 / 1493, 4,194,304 x 64 3587 / 3653), not below (65,536 x 64 with all
-//     levels in FP32 285 / 282).
-static bool precision_level_fp32(int n, int64_t ntiles, int vec) {
-    const bool few = ntiles <= 128;
-    return n > 32 ? !few : few || (n < 32 && vec);
+// Whether a level of the precision form takes the FP32 Q assembly: its CTA has
+// no TMEM to allocate, no operands to split and no padded columns to multiply,
+// and its error is the smaller one.  Whole calls, us with tcgen05 on every level
+// over us with FP32 on every level, by rows and base and leading dimension on
+// (vec) or off 16 bytes:
+//   columns below the tile's width: FP32.  1.05 .. 1.48 with vec at 4 to 56
+//     columns and 512 to 2,000,000 rows.  Without vec 1.00 .. 1.39, but up to 32
+//     columns the level alone is the slower one where it is large and nearly as
+//     wide as its tile (tcgen05 there over FP32 there 1.03 at 256 tiles of 31
+//     columns, 1.00 at 391, 0.96 at 512 and 3907; 20 columns 1.05 .. 1.03, 12 and
+//     24 1.03 .. 0.99): tcgen05 above 384 tiles from two thirds of the width on.
+//   16 and 32 columns fill their tiles: FP32 on levels of up to 128 tiles (16
+//     columns 1.05 .. 1.13 with vec, 1.01 .. 1.07 without; 32 columns 1.04 ..
+//     1.09, 1.01 .. 1.04).  Above, 16 columns with vec still 1.01 .. 1.06, but
+//     without 1.03 falling to 0.95 at 1,000,000 rows; 32 columns 1.05 .. 0.995
+//     and 1.03 .. 0.94, equal near 300 and 150 tiles: tcgen05.
+//   64 columns: tcgen05 (0.986 .. 1.000 with vec to 200,000 rows, 0.95 .. 0.98
+//     without), FP32 with vec above 512 tiles (1.014 .. 1.015 from 400,000 rows).
+static bool precision_level_fp32(int n, int nmax, int64_t ntiles, int vec) {
+    if (n < nmax) return vec || nmax == 64 || ntiles <= 384 || 3 * n < 2 * nmax;
+    if (n == 64) return vec && ntiles > 512;
+    return ntiles <= 128 || (n == 16 && vec);
 }
 
 size_t tsqr_precision_workspace(int64_t m, int64_t n, PrecFlags f) {
@@ -511,7 +519,7 @@ tsqr_status tsqr_precision(int64_t m, int64_t n, float* A, int64_t lda, float* R
         ap.P = (l == L - 1) ? nullptr : lv[l + 1].M;
         ap.ldp = (l == L - 1) ? 0 : lv[l + 1].ld;
         ap.vec = (lv[l].ld % 4 == 0 && (reinterpret_cast<uintptr_t>(lv[l].M) % 16) == 0) ? 1 : 0;
-        if (precision_level_fp32((int)n, lv[l].ntiles, ap.vec)) {
+        if (precision_level_fp32((int)n, c.nmax, lv[l].ntiles, ap.vec)) {
             c.ks.apply(ap, (int)lv[l].ntiles, s);
         } else if (!tc_apply_level(ap, c.nmax, c.rows, err, s)) {
             return TSQR_ERR_UNSUPPORTED;
@@ -686,16 +694,16 @@ tsqr_status tsqr_host(int64_t m, int64_t n, const T* hA, int64_t lda, T* hQ, int
         ap.stack = l > 0;
         ap.P = (l == L - 1) ? nullptr : lv[l + 1].M + t0 * n;
         ap.ldp = (l == L - 1) ? 0 : lv[l + 1].ld;
+        constexpr int ve = 16 / sizeof(T);
+        ap.vec = (ap.ld % ve == 0 && (reinterpret_cast<uintptr_t>(ap.M) % 16) == 0) ? 1 : 0;
         if constexpr (sizeof(T) == 4) {
-            if (tc) {
-                ap.vec = 0;
+            // by the whole level, as for a matrix in device memory
+            if (tc && !precision_level_fp32((int)n, nmax, lv[l].ntiles, ap.vec)) {
                 if (!tc_apply_level(ap, nmax, (int)rows, err, s)) return false;
                 log_launch(kTagTc + l, s);
                 return true;
             }
         }
-        constexpr int ve = 16 / sizeof(T);
-        ap.vec = (ap.ld % ve == 0 && (reinterpret_cast<uintptr_t>(ap.M) % 16) == 0) ? 1 : 0;
         ks.apply(ap, (int)std::min<int64_t>(cnt, 1 << 30), s);
         log_launch(kTagApply + l, s);
         return true;
