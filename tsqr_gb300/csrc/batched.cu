@@ -140,9 +140,10 @@ __global__ void __launch_bounds__(256, ApplyF32<NMAX, ROWS>::kResident)
     apply_tile_f32<NMAX, ROWS>(apply_sm, w.M + row0, w.ld, ht, w.n, w.P ? w.P + lt * w.n : nullptr, w.ldp, vec);
 }
 
-// Per-class configuration; tile heights and kernels equal those of the
-// single-problem path (tsqr.cu), so a problem's tree and arithmetic are the
-// same either way.
+// Per-class configuration.  Tile heights equal those of the single-problem path
+// (tsqr.cu), so a problem's tree and signs are the same either way.  The factor
+// kernel may differ (a launch's tiles in all decide, not the problem's own: see
+// SplitCls), and with it the rounding.
 struct ClassCfg {
     int nmax, rows;
     int factor_per_sm;  // resident factor CTAs per SM
