@@ -82,14 +82,14 @@ template <int NMAX, int NT, int RPT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) batched_factor(const __grid_constant__ FactorTable tab) {
     pdl_begin();
     constexpr int B = NT * RPT;
-    __shared__ FactorSmem<float, NMAX, NT, false> S;
+    __shared__ FactorSmem<NMAX, NT> S;
     for (int64_t t = blockIdx.x; t < tab.total; t += gridDim.x) {
         const int i = find_item(tab.it, tab.count, t);
         const FactorItem& w = tab.it[i];
         const int64_t lt = t - w.tile0;
         const int64_t row0 = lt * B;
         const int ht = (int)((w.h - row0) < B ? (w.h - row0) : B);
-        factor_tile<float, NMAX, NT, RPT, false>(S, w.M + row0, w.ld, ht, w.n, w.Rout + lt * w.n, w.ldr);
+        factor_tile<NMAX, NT, RPT>(S, w.M + row0, w.ld, ht, w.n, w.Rout + lt * w.n, w.ldr);
     }
 }
 

@@ -43,26 +43,12 @@ struct TransposeRound {
     }
 };
 
-// Reduce NV partials across the warp and store the warp's NV sums to row[].
-template <typename T, int NV>
-__device__ __forceinline__ void warp_reduce_to_smem(T (&p)[NV], T* row, int lane) {
-    TransposeRound<NV, 16>::run(p, lane);
-    if constexpr (NV >= 32) {
-        constexpr int K = NV / 32;
-#pragma unroll
-        for (int k = 0; k < K; ++k) row[lane * K + k] = p[k];
-    } else {
-        constexpr int G = 32 / NV;
-        if ((lane % G) == 0) row[lane / G] = p[0];
-    }
-}
-
-// Same result as warp_reduce_to_smem, through a per-warp shared-memory
-// transpose instead of shuffles: every lane stores its NV partials as one
+// Reduce NV partials across the warp and store the warp's NV sums to row[],
+// through a per-warp shared-memory transpose: every lane stores its NV partials as one
 // padded row (16-byte stores), then lane l sums column l (and l + 32 for
 // NV = 64).  The row stride NV + 4 keeps both the row stores and the column
 // loads free of bank conflicts.  About 8 + 32 + 31 instructions per lane for
-// NV = 32 instead of 31 shuffles, 31 adds and 62 selects.  FP32 only.
+// NV = 32 instead of 31 shuffles, 31 adds and 62 selects of a shuffle reduction.
 template <int NV>
 __host__ __device__ constexpr int xpose_stride() {
     return NV + 4;

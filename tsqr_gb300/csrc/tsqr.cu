@@ -135,13 +135,13 @@ void apply_level(const ApplyParams<T>& p, cudaStream_t s) {
         apply_level_f64<NMAX, ROWS>(p, s);
 }
 
-template <typename T, int NMAX, int NT, int RPT, int MINB>
+template <int NMAX, int NT, int RPT, int MINB>
 struct TileCfg {
     static constexpr int kRows = NT * RPT;
-    static void factor(const FactorParams<T>& p, int grid, cudaStream_t s) {
-        launch_pdl(factor_tiles<T, NMAX, NT, RPT, MINB, false>, dim3(grid), dim3(NT), 0, s, p);
+    static void factor(const FactorParams<float>& p, int grid, cudaStream_t s) {
+        launch_pdl(factor_tiles<NMAX, NT, RPT, MINB>, dim3(grid), dim3(NT), 0, s, p);
     }
-    static void apply(const ApplyParams<T>& p, int, cudaStream_t s) { apply_level<T, NMAX, kRows>(p, s); }
+    static void apply(const ApplyParams<float>& p, int, cudaStream_t s) { apply_level<float, NMAX, kRows>(p, s); }
 };
 
 // Factor on column-split tiles (factor_split_tiles: NMAX/CW warps per
@@ -243,7 +243,7 @@ KernelSet<float> pick(float*, int n) {
     // n = 16: 0.20 vs 0.49 ms; n = 32: 0.72 vs 0.98 ms.  2,097,152 x 64: two
     // panels (factor_panel_tiles) 1.07 ms, column-split in one 1.64 ms.
     // n = 64 keeps 512-row tiles (256-row tiles double the stacked-R level).
-    if (n <= 8) return make_set<TileCfg<float, 8, 256, 4, 3>, float>();
+    if (n <= 8) return make_set<TileCfg<8, 256, 4, 3>, float>();
     if (n <= 16) return make_set<SplitCfg<float, 16, 4, 16, 4>, float>();
     if (n <= 32) return make_set<SplitCfg<float, 32, 4, 16, 2>, float>();
     if (n <= 64) return make_set<WideCfg, float>();

@@ -23,8 +23,7 @@
 //   reduction also yields column j of V^T V, from which T is formed once per
 //   tile: row i of T depends only on row i (T(i,j) = -tau_j sum_k T(i,k)
 //   S(k,j)), so thread i builds it alone.  R goes to the next level's rows
-//   [t*n, t*n+n), or to the caller's R at the root.  With NORM64 the norm,
-//   beta and tau are computed in FP64.
+//   [t*n, t*n+n), or to the caller's R at the root.
 //
 // apply_tiles_f32 (and apply_f64_tiles in tile_f64.cuh): down-sweep
 //   (kernelQR.h:397-492 and tsgemm_tsqr, TallShinnyQR.h:11-74): given the parent's n x n block B_t (the root uses
@@ -89,22 +88,20 @@ struct SCols {
     __align__(16) T c[NMAX][LD];
 };
 
-// Shared memory of one factor CTA.
-template <typename T, int NMAX, int NT, bool NORM64>
+// Shared memory of one factor_tiles CTA.
+template <int NMAX, int NT>
 struct FactorSmem {
     static constexpr int NW = NT / 32;
-    using N64 = typename std::conditional<NORM64, double, T>::type;
-    N64 s_part[NW];
-    T s_alpha;
-    T red[NW][NMAX];
-    __align__(16) T wfin[NW][NMAX];
-    SCols<T, NMAX> Sc;
-    T Tsh[NMAX][NMAX + 1];
-    T tau_sh[NMAX];
-    T rdiag[NMAX];
-    // per-warp transpose scratch of the FP32 dot-product reduction
-    __align__(16) float xpose[std::is_same<T, float>::value ? NW : 1]
-                             [std::is_same<T, float>::value ? 32 * xpose_stride<NMAX>() : 4];
+    float s_part[NW];
+    float s_alpha;
+    float red[NW][NMAX];
+    __align__(16) float wfin[NW][NMAX];
+    SCols<float, NMAX> Sc;
+    float Tsh[NMAX][NMAX + 1];
+    float tau_sh[NMAX];
+    float rdiag[NMAX];
+    // per-warp transpose scratch of the dot-product reduction
+    __align__(16) float xpose[NW][32 * xpose_stride<NMAX>()];
 };
 
 // Row i of the compact-WY factor T of a tile: T(i,i) = tau_i and
@@ -143,13 +140,12 @@ __device__ __forceinline__ void t_factor_row(const SCols<T, NMAX>& S, const T* t
 // (leading dimension ld), factored in place (V below the diagonal, T in the
 // top block's upper triangle); its n x n R goes to Rt (leading dimension
 // ldr).  Called by every thread of the CTA.
-template <typename T, int NMAX, int NT, int RPT, bool NORM64>
-__device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, T* tile, int64_t ld, int ht, int n,
-                                            T* Rt, int64_t ldr) {
+template <int NMAX, int NT, int RPT>
+__device__ __forceinline__ void factor_tile(FactorSmem<NMAX, NT>& S, float* tile, int64_t ld, int ht, int n, float* Rt,
+                                            int64_t ldr) {
     constexpr int NW = NT / 32;
     constexpr int U = 4;  // columns per unrolled group
     static_assert(NT >= NMAX && NT % 32 == 0 && NMAX % U == 0, "bad tile configuration");
-    using N64 = typename FactorSmem<T, NMAX, NT, NORM64>::N64;
     auto& s_part = S.s_part;
     auto& s_alpha = S.s_alpha;
     auto& red = S.red;
@@ -170,13 +166,13 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
         // are the group's columns) and position NMAX - U*g + k holds the
         // finished reflector v_k.  All register indices stay compile-time
         // while the code holds U column steps instead of NMAX.
-        T y[RPT][NMAX];
+        float y[RPT][NMAX];
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
             const int r = tid + NT * i;
 #pragma unroll
             for (int c = 0; c < NMAX; ++c)
-                y[i][c] = (r < ht && c < n) ? tile[r + c * ld] : T(0);
+                y[i][c] = (r < ht && c < n) ? tile[r + c * ld] : 0.f;
         }
 
 #pragma unroll 1
@@ -191,59 +187,54 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
                     // Row slots i >= 1 hold rows >= NT >= NMAX > j, so only
                     // slot 0 needs the row-versus-diagonal tests below.
                     // (a) sigma^2 = ||x(j+1:, j)||^2 and alpha = x(j, j)
-                    N64 s = 0;
+                    float s = 0;
 #pragma unroll
                     for (int i = 0; i < RPT; ++i) {
                         const int r = tid + NT * i;
-                        if (i > 0 || r > j) s += (N64)y[i][u] * (N64)y[i][u];
+                        if (i > 0 || r > j) s += y[i][u] * y[i][u];
                         if (i == 0 && r == j) s_alpha = y[i][u];
                     }
                     s = warp_sum(s);
                     if (lane == 0) s_part[warp] = s;
                     __syncthreads();
-                    N64 sigma2 = 0;
+                    float sigma2 = 0;
 #pragma unroll
                     for (int w = 0; w < NW; ++w) sigma2 += s_part[w];
-                    const N64 alpha = s_alpha;
-                    N64 beta, tau, scale;
-                    if (sigma2 == N64(0)) {
+                    const float alpha = s_alpha;
+                    float beta, tau, scale;
+                    if (sigma2 == 0.f) {
                         tau = 0;
                         beta = alpha;
                         scale = 0;
                     } else {
-                        const N64 nrm = sqrt(alpha * alpha + sigma2);
-                        beta = (alpha >= N64(0)) ? -nrm : nrm;
+                        const float nrm = sqrt(alpha * alpha + sigma2);
+                        beta = (alpha >= 0.f) ? -nrm : nrm;
                         // reciprocal-multiply (round-to-nearest reciprocal)
                         // keeps the slow division path off the column chain
                         tau = (beta - alpha) * recip(beta);
                         scale = recip(alpha - beta);
                     }
-                    const T taut = (T)tau;
-                    const T scalet = (T)scale;
                     // (b) v_j below the diagonal (v_j(j) = 1 implicitly), then
                     // v_j . y[c] for every other position: trailing columns
                     // (update) and finished reflectors (column j of V^T V)
 #pragma unroll
                     for (int i = 0; i < RPT; ++i) {
                         const int r = tid + NT * i;
-                        if (i > 0 || r > j) y[i][u] *= scalet;
+                        if (i > 0 || r > j) y[i][u] *= scale;
                     }
                     // v of slot 0: 0 above the diagonal, 1 on it
-                    const T v0 = (tid > j) ? y[0][u] : ((tid == j) ? T(1) : T(0));
-                    T pc[NMAX];
+                    const float v0 = (tid > j) ? y[0][u] : ((tid == j) ? 1.f : 0.f);
+                    float pc[NMAX];
 #pragma unroll
-                    for (int c = 0; c < NMAX; ++c) pc[c] = (c != u) ? v0 * y[0][c] : T(0);
+                    for (int c = 0; c < NMAX; ++c) pc[c] = (c != u) ? v0 * y[0][c] : 0.f;
 #pragma unroll
                     for (int i = 1; i < RPT; ++i) {
-                        const T v = y[i][u];
+                        const float v = y[i][u];
 #pragma unroll
                         for (int c = 0; c < NMAX; ++c)
                             if (c != u) pc[c] += v * y[i][c];
                     }
-                    if constexpr (std::is_same<T, float>::value)
-                        warp_reduce_to_smem_x<NMAX>(pc, red[warp], xpose[warp], lane);
-                    else
-                        warp_reduce_to_smem<T, NMAX>(pc, red[warp], lane);
+                    warp_reduce_to_smem_x<NMAX>(pc, red[warp], xpose[warp], lane);
                     __syncthreads();
                     // (c) every warp sums the NW partials itself; positions
                     // that are not trailing columns get a zero coefficient, so
@@ -254,10 +245,10 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
                         for (int kk = 0; kk < K; ++kk) {
                             const int idx = (NMAX >= 32) ? lane * K + kk : lane;
                             if (idx < NMAX) {
-                                T a = 0;
+                                float a = 0;
 #pragma unroll
                                 for (int w = 0; w < NW; ++w) a += red[w][idx];
-                                wfin[warp][idx] = (idx > u && idx < live) ? a : T(0);
+                                wfin[warp][idx] = (idx > u && idx < live) ? a : 0.f;
                                 if (warp == 0) {
                                     const int k = (idx >= past0) ? idx - past0 : ((idx < u) ? base + idx : -1);
                                     if (k >= 0) Sc[j][k] = a;
@@ -265,19 +256,19 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
                             }
                         }
                         if (tid == 0) {
-                            tau_sh[j] = taut;
-                            rdiag[j] = (T)beta;
+                            tau_sh[j] = tau;
+                            rdiag[j] = beta;
                         }
                     }
                     __syncwarp();
                     // (d) trailing update x_c -= tau (v^T x_c) v (v = 0 above
                     // the diagonal, coefficient 0 off the trailing columns)
-                    T wr[NMAX];
+                    float wr[NMAX];
 #pragma unroll
                     for (int c = 0; c < NMAX; ++c) wr[c] = wfin[warp][c];
 #pragma unroll
                     for (int i = 0; i < RPT; ++i) {
-                        const T tv = taut * ((i > 0) ? y[i][u] : v0);
+                        const float tv = tau * ((i > 0) ? y[i][u] : v0);
 #pragma unroll
                         for (int c = u + 1; c < NMAX; ++c) y[i][c] -= tv * wr[c];
                     }
@@ -286,7 +277,7 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
             // rotate every register row left by U
 #pragma unroll
             for (int i = 0; i < RPT; ++i) {
-                T keep[U];
+                float keep[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) keep[u] = y[i][u];
 #pragma unroll
@@ -301,8 +292,8 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
         // T(i,j) = -tau_j sum_{k=i}^{j-1} T(i,k) S(k,j) for j > i.
         if (tid < n) {
             const int i = tid;
-            T trow[NMAX];
-            t_factor_row<T, NMAX>(S.Sc, tau_sh, i, n, trow);
+            float trow[NMAX];
+            t_factor_row<float, NMAX>(S.Sc, tau_sh, i, n, trow);
 #pragma unroll
             for (int j = 0; j < NMAX; ++j) Tsh[i][j] = trow[j];
         }
@@ -315,8 +306,8 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
             for (int c = 0; c < NMAX; ++c) {
                 const int k = (c + shift) % NMAX;
                 if (k < n) {
-                    T v = (k > r) ? y[0][c] : ((k == r) ? rdiag[r] : T(0));
-                    if (r >= ht) v = T(0);
+                    float v = (k > r) ? y[0][c] : ((k == r) ? rdiag[r] : 0.f);
+                    if (r >= ht) v = 0.f;
                     Rt[r + k * ldr] = v;
                 }
             }
@@ -337,16 +328,16 @@ __device__ __forceinline__ void factor_tile(FactorSmem<T, NMAX, NT, NORM64>& S, 
     }
 }
 
-template <typename T, int NMAX, int NT, int RPT, int MINB, bool NORM64>
-__global__ void __launch_bounds__(NT, MINB) factor_tiles(FactorParams<T> p) {
+template <int NMAX, int NT, int RPT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) factor_tiles(FactorParams<float> p) {
     pdl_begin();
     clear_status(p);
     constexpr int B = NT * RPT;
-    __shared__ FactorSmem<T, NMAX, NT, NORM64> S;
+    __shared__ FactorSmem<NMAX, NT> S;
     for (int64_t t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
         const int64_t row0 = t * B;
         const int ht = (int)((p.h - row0) < B ? (p.h - row0) : B);
-        factor_tile<T, NMAX, NT, RPT, NORM64>(S, p.M + row0, p.ld, ht, p.n, p.Rout + t * p.n, p.ldr);
+        factor_tile<NMAX, NT, RPT>(S, p.M + row0, p.ld, ht, p.n, p.Rout + t * p.n, p.ldr);
     }
 }
 
