@@ -65,3 +65,17 @@ def test_fp64_columns_of_very_different_norms(orc, cuda, tg, small, large, n):
     e = [0] * n
     e[n // 4], e[n // 2 + 1] = small, large
     check(orc, tg, 3000, n, e, 9)
+
+
+@pytest.mark.parametrize("n", [8, 16, 24, 32])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 1e200])
+def test_fp64_a_bad_last_column_leaves_the_others_of_r(orc, cuda, tg, bad, n):
+    """An element that makes the last column's norm infinite or NaN: the columns
+    of R before it are formed without it and keep every bit."""
+    m = 5000
+    A = orc.fill_uniform(m, n, np.float64, seed=10)
+    _, R0 = run(tg, A)
+    A[m - 1, n - 1] = bad
+    _, R = run(tg, A)
+    assert np.array_equal(R[:, :n - 1], R0[:, :n - 1])
+    assert not np.isfinite(R[:, n - 1]).all()
