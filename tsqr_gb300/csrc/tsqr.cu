@@ -449,11 +449,12 @@ bool tc_apply_level(const ApplyParams<float>& p, int nmax, int rows, int* err, c
 //     1.09, 1.01 .. 1.04).  Above, 16 columns with vec still 1.01 .. 1.06, but
 //     without 1.03 falling to 0.95 at 1,000,000 rows; 32 columns 1.05 .. 0.995
 //     and 1.03 .. 0.94, equal near 300 and 150 tiles: tcgen05.
-//   64 columns: tcgen05 (0.986 .. 1.000 with vec to 200,000 rows, 0.95 .. 0.98
-//     without), FP32 with vec above 512 tiles (1.014 .. 1.015 from 400,000 rows).
+//   64 columns: FP32 above 128 tiles, for its error (200,000 x 64 backward 3.6e-7
+//     against 4.5e-7; 0.99 .. 1.015 with vec, 0.96 .. 0.98 without), tcgen05 on the
+//     smaller levels (0.986 .. 0.998, 0.95 .. 0.98).
 static bool precision_level_fp32(int n, int nmax, int64_t ntiles, int vec) {
     if (n < nmax) return vec || nmax == 64 || ntiles <= 384 || 3 * n < 2 * nmax;
-    if (n == 64) return vec && ntiles > 512;
+    if (n == 64) return ntiles > 128;
     return ntiles <= 128 || (n == 16 && vec);
 }
 
