@@ -31,7 +31,8 @@ namespace {
 
 constexpr int kTile = 64;    // output tile edge of gemm_nn (rows)
 constexpr int kTnTile = 32;  // output tile edge of gemm_tn_partial
-constexpr int kKt = 16;    // k step through shared memory
+constexpr int kKt = 16;      // k step through shared memory
+constexpr int kTnBlock = 256;  // rows that gemm_tn_partial sums on their own
 
 // P_z (M x N, ld M) = sum over k in chunk z of A(k, i) * B(k, j);
 // A is K x M, B is K x N, both column-major.
@@ -40,7 +41,10 @@ constexpr int kKt = 16;    // k step through shared memory
 // padding; the loads for 2 x 2 outputs per thread cost nothing beside it.
 // 27,648 rows, us: 32 x 32 264 -> 55, the three products of a 128-column qr
 // 799 -> 305, against a 64 x 64 tile with 4 x 4 outputs in chunks of at least
-// 256 rows.
+// 256 rows.  A chunk may be long (wide nodes fill the SMs with one each), so its
+// products are summed in blocks of 256 rows: a running sum of k terms has a
+// rounding error that grows with k, and one of 1100 rows cost a 1100 x 1024 qr a
+// quarter of its orthogonality.
 template <typename T>
 __global__ void __launch_bounds__(256) gemm_tn_partial(int M, int N, int64_t K, const T* __restrict__ A,
                                                        int64_t lda, const T* __restrict__ B, int64_t ldb,
@@ -54,7 +58,7 @@ __global__ void __launch_bounds__(256) gemm_tn_partial(int M, int N, int64_t K, 
     const int i0 = blockIdx.x * kTnTile, j0 = blockIdx.y * kTnTile;
     const int64_t kbeg = (int64_t)blockIdx.z * kchunk;
     const int64_t kend = min(K, kbeg + kchunk);
-    T acc[R][R] = {};
+    T sum[R][R] = {};
     // the next k step's elements are loaded into registers while the current
     // one is multiplied out of shared memory
     T ra[L], rb[L];
@@ -69,30 +73,38 @@ __global__ void __launch_bounds__(256) gemm_tn_partial(int M, int N, int64_t K, 
         }
     };
     if (kbeg < kend) fetch(kbeg);
-    for (int64_t k0 = kbeg; k0 < kend; k0 += kKt) {
+    for (int64_t kb = kbeg; kb < kend; kb += kTnBlock) {
+        T acc[R][R] = {};
+        const int64_t ke = min(kend, kb + kTnBlock);
+        for (int64_t k0 = kb; k0 < ke; k0 += kKt) {
 #pragma unroll
-        for (int e = 0; e < L; ++e) {
-            const int idx = tid + 256 * e;
-            const int kk = idx % kKt, col = idx / kKt;
-            As[kk][col] = ra[e];
-            Bs[kk][col] = rb[e];
-        }
-        __syncthreads();
-        if (k0 + kKt < kend) fetch(k0 + kKt);
-#pragma unroll
-        for (int kk = 0; kk < kKt; ++kk) {
-            T a[R], b[R];
-#pragma unroll
-            for (int u = 0; u < R; ++u) {
-                a[u] = As[kk][ty * R + u];
-                b[u] = Bs[kk][tx * R + u];
+            for (int e = 0; e < L; ++e) {
+                const int idx = tid + 256 * e;
+                const int kk = idx % kKt, col = idx / kKt;
+                As[kk][col] = ra[e];
+                Bs[kk][col] = rb[e];
             }
+            __syncthreads();
+            if (k0 + kKt < kend) fetch(k0 + kKt);
 #pragma unroll
-            for (int u = 0; u < R; ++u)
+            for (int kk = 0; kk < kKt; ++kk) {
+                T a[R], b[R];
 #pragma unroll
-                for (int v = 0; v < R; ++v) acc[u][v] += a[u] * b[v];
+                for (int u = 0; u < R; ++u) {
+                    a[u] = As[kk][ty * R + u];
+                    b[u] = Bs[kk][tx * R + u];
+                }
+#pragma unroll
+                for (int u = 0; u < R; ++u)
+#pragma unroll
+                    for (int v = 0; v < R; ++v) acc[u][v] += a[u] * b[v];
+            }
+            __syncthreads();
         }
-        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < R; ++u)
+#pragma unroll
+            for (int v = 0; v < R; ++v) sum[u][v] += acc[u][v];
     }
     T* Pz = P + (int64_t)blockIdx.z * M * N;
 #pragma unroll
@@ -100,7 +112,7 @@ __global__ void __launch_bounds__(256) gemm_tn_partial(int M, int N, int64_t K, 
 #pragma unroll
         for (int v = 0; v < R; ++v) {
             const int i = i0 + ty * R + u, j = j0 + tx * R + v;
-            if (i < M && j < N) Pz[i + (int64_t)j * M] = acc[u][v];
+            if (i < M && j < N) Pz[i + (int64_t)j * M] = sum[u][v];
         }
 }
 
