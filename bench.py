@@ -57,12 +57,12 @@ sys.path.insert(0, ROOT)
 METRIC = "QR TFLOP/s & % roofline, tensor-core vs plain FP32 at equal FP64-oracle error"
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the
-# level-0 kernels at 4,194,304 x 32: one ncu --set full capture of each kernel
-# at 2,097,152 rows (factor 494.6 MB, tensor-core apply 492.8 MB, CUDA-core
-# apply 492.2 MB), scaled by the tile count (x2).
-TRAFFIC = {(4194304, 32, "factor_level0"): 2 * 493.6e6,
-           (4194304, 32, "tc_level0"): 2 * 492.5e6,
-           (4194304, 32, "apply_level0"): 2 * 492.2e6}
+# level-0 kernels at 4,194,304 x 32: an ncu capture of each kernel at 2,097,152
+# rows (factor_panel_tiles_tma 493.5 MB, mean of two launches; tc_apply_tiles
+# 489.9 MB; apply_tiles_f32 490.1 MB), scaled by the tile count (x2).
+TRAFFIC = {(4194304, 32, "factor_level0"): 2 * 493.5e6,
+           (4194304, 32, "tc_level0"): 2 * 489.9e6,
+           (4194304, 32, "apply_level0"): 2 * 490.1e6}
 TRAFFIC_SOURCE = "ncu capture at 2,097,152 rows, x2 for the tile count"
 
 

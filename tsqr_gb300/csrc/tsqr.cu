@@ -355,9 +355,10 @@ tsqr_status tsqr_plain(int64_t m, int64_t n, T* A, int64_t lda, T* R, int64_t ld
 
 // ---------------------------------------------------------------------------
 // Precision form (FP32 entry points): the tile factorisation stays FP32 on
-// CUDA cores; every Q assembly of the down-sweep runs on tcgen05 in TF32x3
-// (tc_apply.cu).  An FP64 root combine (the last level converted to double
-// and factored by the FP64 tree) is built in but switched off (kRoot64).
+// CUDA cores; the Q assembly of a level runs on tcgen05 in TF32x3
+// (tc_apply.cu) or in FP32, as precision_level_fp32 says.  With
+// tsqr_opts.fp64_root the last level is converted to double and factored by
+// the FP64 tree.
 // Workspace: [status word (256 B) | level matrices | FP64 root copy | FP64
 // root-tree workspace].
 // ---------------------------------------------------------------------------

@@ -26,11 +26,12 @@
 //   [t*n, t*n+n), or to the caller's R at the root.
 //
 // apply_tiles_f32 (and apply_f64_tiles in tile_f64.cuh): down-sweep
-//   (kernelQR.h:397-492 and tsgemm_tsqr, TallShinnyQR.h:11-74): given the parent's n x n block B_t (the root uses
-//   B = I), the tile's final Q is (I - V T V^T) [B_t; 0] = [B_t; 0] - V W,
-//   W = T (V_top^T B_t).  W needs only the tile's top block, so the bulk is a
-//   reduction-free (B x n)(n x n) product streamed as n rank-1 updates of
-//   each thread's rows; Q overwrites the tile in place.
+//   (kernelQR.h:397-492 and tsgemm_tsqr, TallShinnyQR.h:11-74): given the
+//   parent's n x n block B_t (the root uses B = I), the tile's final Q is
+//   (I - V T V^T) [B_t; 0] = [B_t; 0] - V W, W = T (V_top^T B_t).  W needs only
+//   the tile's top block, so the bulk is a reduction-free (B x n)(n x n)
+//   product, in chunks of rows that pass through shared memory, 4 rows x 4 or 8
+//   columns per thread; Q overwrites the tile in place.
 //
 // Rows of the last tile past the matrix end are treated as zero rows: they
 // never change, never enter a dot product and are never stored.
@@ -695,6 +696,16 @@ __device__ __forceinline__ int split_steps(SplitFactorSmem<T, NMAX, CW, RPT>& S,
     return shift;
 }
 
+// One tile: ht rows of n columns at `tile` (leading dimension ld), its R to
+// Rt (leading dimension ldr).  A kernel whose registers are full keeps it in
+// shared memory, from which it is read again after the column steps.
+template <typename T>
+struct TileDesc {
+    T* tile;
+    T* Rt;
+    int64_t ld, ldr;
+    int ht, n;
+};
 // VECV: publish the reflector in the 16-byte vector layout (VbufLayout).
 // Off for the 64-column tile and for the batched kernels, whose registers
 // leave no room for the aligned quads it needs (more spills with it).
@@ -707,16 +718,6 @@ __device__ __forceinline__ int split_steps(SplitFactorSmem<T, NMAX, CW, RPT>& S,
 // NMAX columns, box h holding rows [256h, 256h + 256) column by column, the
 // rows past the level's end and the columns past n already zero.  `loaded`
 // runs once every thread holds its values.
-// One tile: ht rows of n columns at `tile` (leading dimension ld), its R to
-// Rt (leading dimension ldr).  A kernel whose registers are full keeps it in
-// shared memory, from which it is read again after the column steps.
-template <typename T>
-struct TileDesc {
-    T* tile;
-    T* Rt;
-    int64_t ld, ldr;
-    int ht, n;
-};
 struct NoHook {
     __device__ __forceinline__ void operator()() const {}
 };
@@ -914,8 +915,8 @@ __device__ __forceinline__ void cp_async_wait_group() {
 // Q assembly of FP32 tiles: Q = [B; 0] - V W with W = T (V_top^T B), in place.
 //
 // A CTA of 256 threads walks a tile in chunks of CH rows, staged in shared
-// memory by asynchronous copies in two buffers: chunk c+1 (or the CTA's next
-// tile's first chunk) is on its way while chunk c is multiplied.  A thread
+// memory by asynchronous copies in two buffers: chunk c+1 is on its way while
+// chunk c is multiplied.  A thread
 // owns 4 rows x TC columns of a chunk; per k it reads one 16-byte vector of V
 // and TC/4 of W.  Lanes that share a column group are adjacent: a warp's
 // 16-byte read of one address by adjacent lanes costs 2.1 cycles of the SM's
@@ -924,7 +925,7 @@ __device__ __forceinline__ void cp_async_wait_group() {
 // W is formed once per tile from chunk 0: the strict lower part of the top
 // block is V_top, its upper triangle T, so both products run over half of the
 // terms and need masks in their diagonal blocks only.  B is staged row-major
-// in the buffer that W takes over, Y in the second chunk buffer (free then).
+// in the buffer that W takes over.
 template <int NMAX, int ROWS>
 struct ApplyF32 {
     static constexpr int NT = 256;
